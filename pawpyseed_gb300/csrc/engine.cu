@@ -493,6 +493,29 @@ static int pageable_access() {
   return v;
 }
 
+// A caller's complex128 array as kernels write it: in place where the device writes pageable host memory
+// and the array lies on 16 bytes (kernels move whole values; a pawpy_c128 needs only 8: an array at 8
+// modulo 16, e.g. a view into a record, would be a misaligned access), else a device buffer that finish()
+// copies out. read: the kernel adds to the array's values.
+struct HostResult {
+  double2 *p;
+  HostResult(pawpy_c128 *host, size_t n, bool read) : p(reinterpret_cast<double2 *>(host)), host_(p) {
+    if (pageable_access() && reinterpret_cast<uintptr_t>(host) % alignof(double2) == 0) return;
+    buf_.alloc(n);
+    if (read) buf_.upload(host_, n);
+    p = buf_.p;
+  }
+  // the results are in the caller's array on return
+  void finish() {
+    buf_.download(host_, buf_.n);
+    sync();
+  }
+
+ private:
+  double2 *host_;
+  DevBuf<double2> buf_;
+};
+
 // Uploads the coefficients of every band into the sorted device layout. Where
 // the device reads pageable host memory through the host page tables (e.g. a
 // Grace-Blackwell node), a kernel reads the band arrays in place; otherwise
@@ -2779,15 +2802,9 @@ void pseudoprojection(pawpy_c128 *projections, pswf_t *wf_ref, pswf_t *wf_proj, 
   ensure_pseudo(ps, flip_spin);
   DevWF &R = *ps.R, &S = *ps.S;
   int f = flip_spin ? 1 : 0;
-  if (pageable_access()) {
-    launch_extract_band(ps.pseudo[f].p, S.nk, host_bands(S), host_bands(R), BAND_NUM,
-                        reinterpret_cast<double2 *>(projections));
-  } else {
-    DevBuf<double2> col((size_t)host_bands(R) * S.nk);
-    launch_extract_band(ps.pseudo[f].p, S.nk, host_bands(S), host_bands(R), BAND_NUM, col.p);
-    col.download(reinterpret_cast<double2 *>(projections), col.n);
-  }
-  sync();
+  HostResult res(projections, (size_t)host_bands(R) * S.nk, false);
+  launch_extract_band(ps.pseudo[f].p, S.nk, host_bands(S), host_bands(R), BAND_NUM, res.p);
+  res.finish();
   PAWPY_API_END()
 }
 
@@ -2823,17 +2840,9 @@ static void do_compensation_terms(pawpy_c128 *overlap, int BAND_NUM, pswf_t *wf_
     col.alloc((size_t)NR * nk);
     launch_extract_band(ps.cross[flip_spin ? 1 : 0].p, nk, NS, NR, BAND_NUM, col.p);
   }
-  // added into the caller's array in place where the device reads and writes host memory
-  double2 *host = reinterpret_cast<double2 *>(overlap);
-  DevBuf<double2> acc;
-  if (!pageable_access()) {
-    acc.alloc((size_t)NR * nk);
-    acc.upload(host, acc.n);
-  }
-  launch_zgemv_f64(ps.A64.p, NR, kc, nk, flip_k(R, 0, flip_spin), B64.p, recip ? col.p : nullptr,
-                   acc.n ? acc.p : host);
-  if (acc.n) acc.download(host, acc.n);
-  sync();
+  HostResult res(overlap, (size_t)NR * nk, true);
+  launch_zgemv_f64(ps.A64.p, NR, kc, nk, flip_k(R, 0, flip_spin), B64.p, recip ? col.p : nullptr, res.p);
+  res.finish();
 }
 
 extern "C" {
@@ -2907,15 +2916,9 @@ int pawpy_gpu_project_all(pawpy_c128 *out, pswf_t *wf_R, pswf_t *wf_S, int num_M
   full_overlap(ps, lists, flip_spin, Smat);
   DevWF &R = *ps.R, &S = *ps.S;
   const int nk = S.nk;
-  if (pageable_access()) {
-    // the device writes the caller's (pageable) array through the host page tables
-    launch_to_host_layout(Smat.p, nk, host_bands(S), host_bands(R), reinterpret_cast<double2 *>(out));
-  } else {
-    DevBuf<double2> o64(Smat.n);
-    launch_to_host_layout(Smat.p, nk, host_bands(S), host_bands(R), o64.p);
-    o64.download(reinterpret_cast<double2 *>(out), o64.n);
-  }
-  sync();
+  HostResult res(out, Smat.n, false);
+  launch_to_host_layout(Smat.p, nk, host_bands(S), host_bands(R), res.p);
+  res.finish();
   return 0;
   PAWPY_API_END(pawpy_gpu_last_error())
 }
@@ -3027,14 +3030,9 @@ static void realspace_overlaps(pswf_t *wf_S, pswf_t *wf_R, const int *fftg, cons
     }
     grid_overlaps(gR.p, nbR, gS.p, ns, ld, n, o.p + (size_t)k0 * ns * nbR);
   }
-  if (pageable_access()) {
-    launch_to_host_layout(o.p, nk, ns, nbR, reinterpret_cast<double2 *>(out), scale);
-  } else {
-    DevBuf<double2> o64(o.n);
-    launch_to_host_layout(o.p, nk, ns, nbR, o64.p, scale);
-    o64.download(reinterpret_cast<double2 *>(out), o64.n);
-  }
-  sync();
+  HostResult res(out, o.n, false);
+  launch_to_host_layout(o.p, nk, ns, nbR, res.p, scale);
+  res.finish();
 }
 
 extern "C" {
