@@ -24,7 +24,9 @@ namespace pawpy {
 
 namespace {
 
+// shared memory of a CTA; pass A keeps its masks (m2, m3) in static shared memory beside the tile
 constexpr size_t kBandSmemCap = 227 * 1024;
+constexpr size_t kPlanesSmemCap = kBandSmemCap - 2 * kTwoMaxRadix * sizeof(uint32_t);
 
 // Threads per CTA at most (chosen per launch, band_threads): with radices up to 10 the steps fit
 // in 64 registers.
