@@ -642,21 +642,4 @@ inline int tune(const std::tuple<int, int, int, int> &key, const std::vector<int
 
 }  // namespace fftfast
 
-// (second, third) lengths of pass A and (first, third) lengths of pass B with
-// compiled kernels
-#define PAWPY_FFT_PAIRS(X) \
-  X(24, 24)                \
-  X(36, 36)                \
-  X(45, 45)                \
-  X(48, 48)                \
-  X(50, 50)                \
-  X(60, 60)                \
-  X(64, 64)                \
-  X(72, 72)                \
-  X(80, 80)                \
-  X(90, 90)                \
-  X(96, 96)                \
-  X(45, 50)                \
-  X(36, 50)
-
 }  // namespace pawpy
