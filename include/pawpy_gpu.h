@@ -453,9 +453,10 @@ int pawpy_gpu_overlap_noalloc(const pawpy_c64 *A, long long lda, const pawpy_c64
  * for work on several threads. With keep_real_space, its real-space
  * wavefunctions stay on the device too (nk nband N1 N2 N3 complex64) and
  * later projections of it onto new sites gather from them instead of
- * transforming again. No counterpart in the reference. Returns 1 when the
- * real-space wavefunctions are resident, 0 when not, -1 with the status set on
- * failure. */
+ * transforming again; on grids without register kernels only while half of the
+ * device's memory stays free. No counterpart in the reference. Returns 1 when
+ * the real-space wavefunctions are resident, 0 when not, -1 with the status set
+ * on failure. */
 int pawpy_gpu_prepare_basis(pswf_t *wf, int keep_real_space);
 
 /* Projection server: requests (a defect wavefunction against a resident

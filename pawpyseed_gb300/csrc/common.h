@@ -114,6 +114,9 @@ void upload_bytes(void *dev, const void *h, size_t bytes);
 void release_staging();
 void dfree(void *p);
 long long device_bytes();
+// Device memory that dmalloc can still give: what the device has free and what the pool in use holds idle;
+// total (may be NULL): the device's memory.
+long long free_device_bytes(long long *total = nullptr);
 
 template <typename T>
 struct DevBuf {

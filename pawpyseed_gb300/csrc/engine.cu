@@ -1561,22 +1561,38 @@ static void project_bands(DevWF &d, const std::vector<const SphereSet *> &sets,
   }
 }
 
-// Real-space wavefunctions of every band, kept on the device (grid sizes with
-// register kernels only); returns whether they were built.
+// Whether real-space wavefunctions of a grid without register kernels are kept on the device: while half of its
+// memory stays free for the projections. (A basis on such a grid was served without them before the grouped form
+// could write them, and 2 spins x 4 k-points x 1,024 bands on 100 x 100 x 108 are 71 GB. On the register
+// kernels' lengths they are kept whatever their size.)
+bool keeps_real_space(long long bytes, long long free_bytes, long long total_bytes) {
+  return bytes <= free_bytes - total_bytes / 2;
+}
+
+// Real-space wavefunctions of every band, kept on the device (grids that a fast form of the band FFT covers);
+// returns whether they were built.
 static bool build_grids(DevWF &d) {
   HostPhase hp("build_grids");
   ensure_coeffs(d);
   const size_t n3d = (size_t)d.N[0] * d.N[1] * d.N[2];
   std::vector<PlaneGeom> geo(d.nk);
   int maxn1 = 0;
+  bool reg = true;  // (order 1: lengths with register kernels)
   for (int k = 0; k < d.nk; k++) {
     DevKpt &q = d.kp[k];
     PlaneGeom g;
     if (!plane_geom(d, k, g)) return false;
     geo[k] = g;
+    reg = reg && (!g.grouped || g.order == 1);
     maxn1 = std::max(maxn1, q.n1);
   }
-  d.grid.alloc((size_t)d.nk * grid_kstride(d));
+  const size_t count = (size_t)d.nk * grid_kstride(d);
+  if (!reg) {
+    long long total = 0;
+    const long long avail = free_device_bytes(&total);
+    if (!keeps_real_space((long long)(count * sizeof(float2)), avail, total)) return false;
+  }
+  d.grid.alloc(count);
   const long long hband = (long long)maxn1 * d.N[1] * d.N[2] * (long long)sizeof(float2);
   const int fbatch = (int)std::max(1LL, std::min<long long>(d.nband, kFftBatchBytes / std::max(1LL, hband)));
   DevBuf<float2> H((size_t)fbatch * maxn1 * d.N[1] * d.N[2]);

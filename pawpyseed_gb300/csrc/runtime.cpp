@@ -398,6 +398,19 @@ void dfree(void *p) {
 
 long long device_bytes() { return rt().bytes; }
 
+long long free_device_bytes(long long *total) {
+  const int dev = device();
+  size_t f = 0, t = 0;
+  PAWPY_CUDA(cudaMemGetInfo(&f, &t));
+  cudaMemPool_t pool = t_pool;
+  if (!pool) PAWPY_CUDA(cudaDeviceGetDefaultMemPool(&pool, dev));
+  uint64_t held = 0, used = 0;
+  PAWPY_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &held));
+  PAWPY_CUDA(cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used));
+  if (total) *total = (long long)t;
+  return (long long)f + (long long)(held - used);
+}
+
 void launch_begin(const char *family) {
   Runtime &r = rt();
   std::lock_guard<std::recursive_mutex> g(r.mu);
