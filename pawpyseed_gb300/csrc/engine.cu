@@ -2411,6 +2411,14 @@ static int choose_splits(int M, int N, int nz, int maxK) {
   return std::min(s, 64);
 }
 
+// Batches of the FP32 contraction in one launch: its grid's z extent is batches x splits (at most 65,535), and
+// their partial sums stay within 256 MiB.
+int grouped_batches(int nz, int splits, long long partial_bytes) {
+  long long g = std::min(nz, 65535 / std::max(1, splits));
+  if (partial_bytes > 0) g = std::min(g, (256LL << 20) / partial_bytes);
+  return (int)std::max(1LL, g);
+}
+
 // What an overlap contraction sums, per k-point (kR = k with the spins swapped under flip):
 //   kPseudo:    <C_R|C_S>
 //   kAugmented: aug_real  <C_R|C_S> + [augmentation columns A32 | B32]
@@ -2990,10 +2998,11 @@ static void grid_overlaps(const float2 *A, int M, const float2 *B, int N, long l
     return;
   }
   // (the split of one batch: the sums do not depend on how many batches are grouped)
-  int splits = choose_splits(M, N, 1, (int)K);
+  const int splits = choose_splits(M, N, 1, (int)K);
+  const int group = grouped_batches(nz, splits, splits > 1 ? (long long)splits * M * N * (long long)sizeof(float2) : 0);
   DevBuf<float2> ws;
-  if (splits > 1) ws.alloc((size_t)splits * nz * M * N);
-  launch_zgemm_f32(db.p, nz, M, N, splits, ws.p);
+  if (splits > 1) ws.alloc((size_t)splits * group * M * N);
+  for (int z = 0; z < nz; z += group) launch_zgemm_f32(db.p + z, std::min(group, nz - z), M, N, splits, ws.p);
 }
 
 // All-electron grids of bands [b0, b0 + nb) at k-point kq, rows of ld >= n3d values (zero past n3d).

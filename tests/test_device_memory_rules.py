@@ -3,6 +3,7 @@ and the calls that follow them."""
 
 import ctypes as C
 
+import numpy as np
 import pytest
 
 GB = 1 << 30
@@ -45,3 +46,29 @@ def test_smaller_basis_on_such_a_grid_keeps_them():
     wf.check_c_projectors()
     assert _lib.lib().pawpy_gpu_prepare_basis(wf.wf_ptr, 1) == 1
     _lib.check()
+
+
+def test_contractions_of_one_launch_stay_within_its_grid_and_workspace():
+    group = rule("_ZN5pawpy15grouped_batchesEiix", C.c_int, C.c_int, C.c_int, C.c_longlong)
+    assert group(8, 64, 64 * 32 * 32 * 8) == 8
+    assert group(1100, 64, 64 * 4 * 8) == 1023  # x 64 splits: 65,472 of 65,535
+    assert group(70000, 1, 0) == 65535
+    assert group(100, 5, 5 * 512 * 512 * 8) == 25
+    assert group(3, 2, 2 * 8192 * 8192 * 8) == 1
+
+
+@pytest.mark.gpu
+def test_realspace_projections_of_more_than_a_thousand_k_points():
+    """1,100 k-points of a contraction in 64 splits: more than one launch's grid holds. Bound: both sides'
+    states in FP32 and the contraction over 32,768 points, 1e-5 as the other real-space projections."""
+    from pawpyseed_gb300.projector import Projector
+    from test_gpu_fft_grouped import wavefunction
+
+    wf, _ = wavefunction((16, 16, 16), 20.0, nk=1100, nband=2, seed=3)
+    basis, _ = wavefunction((16, 16, 16), 20.0, nk=1100, nband=3, seed=3)
+    out = Projector(wf, basis, method="realspace").project_all()
+    vol, n3 = abs(np.linalg.det(wf.structure.lattice)), 32**3
+    for k in (0, 600, 1022, 1023, 1099):
+        S = np.array([wf.get_state_realspace(b, k, 0, dim=(32, 32, 32)).ravel() for b in range(2)])
+        R = np.array([basis.get_state_realspace(b, k, 0, dim=(32, 32, 32)).ravel() for b in range(3)])
+        assert np.abs(out[:, k::1100] - S @ R.conj().T * vol / n3).max() <= 1e-5
