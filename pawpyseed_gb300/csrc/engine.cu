@@ -17,6 +17,7 @@
 #include <complex>
 #include <exception>
 #include <map>
+#include <limits>
 #include <memory>
 #include <mutex>
 #include <numeric>
@@ -110,6 +111,7 @@ struct AeTables {
   DevBuf<float2> tw[3], tw2[3];
   // the plane waves of each k-point as rows of this grid (rs_fft.cu), built when first asked for
   struct Rows {
+    int sparse = -1;  // rs_sparse, once known
     bool built = false;
     DevBuf<int> row_start, row_of, off_y, off_x;
     DevBuf<unsigned short> col_pos;
@@ -2124,6 +2126,18 @@ static void do_overlap_setup_recip(pswf_t *wf_R, pswf_t *wf_S, const int *labels
 
 // ============================================================= all-electron real-space wavefunctions
 
+// How many of `want` equal pieces of scratch (band grids, k-points) a real-space call holds at once, at least one:
+// what a quarter of the free device memory and `cap` hold, or 256 MiB if that is more.
+constexpr long long kScratchBytes = 256LL << 20;
+int scratch_pieces(long long want, long long bytes_each, long long cap, long long free_bytes) {
+  const long long budget = std::max(kScratchBytes, std::min(cap, free_bytes / 4));
+  return (int)std::max(1LL, std::min(want, budget / std::max(1LL, bytes_each)));
+}
+// (the free memory is asked for where the pieces need more than that)
+static int scratch_count(long long want, long long bytes_each, long long cap) {
+  return scratch_pieces(want, bytes_each, cap, want * bytes_each <= kScratchBytes ? 0 : free_device_bytes());
+}
+
 // The real-space sphere tables of d's sites on grid N (built once per grid and site list).
 static AeTables &ae_tables(DevWF &d, const int *N, const int *labels, const double *coords) {
   PAWPY_REQUIRE(d.tables_ready, "real-space wavefunctions need setup_projections first");
@@ -2318,13 +2332,25 @@ static const RsPlan &rs_plan(DevWF &d, AeTables &t, int kq) {
   return o.plan;
 }
 
+// whether rs_fft.cu transforms k-point q on grid N: plane waves that fall on one another (a grid smaller than the
+// sphere) and lengths that do not group keep the whole-grid form
+static bool rs_sparse(DevWF &d, AeTables &t, int kq) {
+  int &v = t.rows[kq].sparse;
+  if (v < 0) v = rs_fft_supported(t.N) && d.kp[kq].n1 <= t.N[0] && rs_rows_distinct(d.kp[kq], t.N);
+  return v;
+}
+
+// scratch of rs_grids per band, at most
+static long long rs_band_bytes(DevWF &d, AeTables &t, int kq) {
+  return rs_sparse(d, t, kq) ? 2LL * std::max(1, d.kp[kq].n1) * t.N[1] * t.N[2] * (long long)sizeof(float2) : 0;
+}
+
 // sum_G C_G exp(i G.r) of bands [b0, b0 + nb) of k-point kq on the grid of t, grid[b stride + cell].
 static void rs_grids(DevWF &d, AeTables &t, int kq, int b0, int nb, float2 *grid, long long stride) {
   DevKpt &q = d.kp[kq];
   const float2 *C = coeffs(d, kq) + (size_t)b0 * q.Wpad;
   const int *N = t.N;
-  // plane waves that fall on one another (a grid smaller than the sphere) keep the whole-grid form
-  if (rs_fft_supported(N) && q.n1 <= N[0] && rs_rows_distinct(q, N)) {
+  if (rs_sparse(d, t, kq)) {
     const RsPlan &pl = rs_plan(d, t, kq);
     DevBuf<float2> Z((size_t)nb * std::max(1, pl.nrows) * N[2]), Y((size_t)nb * std::max(1, pl.n1) * N[1] * N[2]);
     const float2 *tw[3] = {t.tw2[0].p, t.tw2[1].p, t.tw2[2].p};
@@ -2347,12 +2373,25 @@ static const float2 *proj_rows(DevWF &d, int kq, int b0) {
   return d.P.p + ((size_t)kq * d.nband + b0) * d.proj.Ptot;
 }
 
-// The Bloch factors of k-point kq on the grid of t (nullptr at Gamma), scale included.
-static const float4 *bloch_table(DevWF &d, AeTables &t, int kq, DevBuf<float4> &buf) {
-  if (kpoint_is_gamma(d.kp[kq])) return nullptr;
-  buf.alloc((size_t)t.N[0] * t.N[1] * t.N[2]);
-  launch_bloch_table(t.N, d.kp[kq].kfrac, std::pow(d.vol, -0.5), buf.p);
-  return buf.p;
+// The Bloch factors of k-point kq on the grid of t (scale included): f(slab) for the whole grid, or for one slab
+// of the first axis after another where the grid's table (16 bytes per cell) would be larger than kScratchBytes. buf keeps
+// the whole grid's for the k-point's other calls.
+template <typename F>
+static void with_bloch(DevWF &d, AeTables &t, int kq, DevBuf<float4> &buf, F &&f) {
+  const int *N = t.N;
+  const long long plane = (long long)N[1] * N[2];
+  const int nx = (int)std::max(1LL, std::min<long long>(N[0], kScratchBytes / (plane * (long long)sizeof(float4))));
+  if (kpoint_is_gamma(d.kp[kq])) {
+    f(BlochSlab{nullptr, 0, N[0]});
+    return;
+  }
+  const bool whole = nx == N[0], built = whole && buf.n;
+  if (!buf.n) buf.alloc((size_t)nx * plane);
+  for (int x0 = 0; x0 < N[0]; x0 += nx) {
+    const BlochSlab slab{buf.p, x0, std::min(nx, N[0] - x0)};
+    if (!built) launch_bloch_table(N, slab, d.kp[kq].kfrac, std::pow(d.vol, -0.5), buf.p);
+    f(slab);
+  }
 }
 
 // All-electron states of bands [b0, b0 + nb) of k-point kq to host x (realspace_state,
@@ -2364,8 +2403,9 @@ static void ae_states(DevWF &d, AeTables &t, int kq, int b0, int nb, pawpy_c128 
   rs_grids(d, t, kq, b0, nb, g.p, n3d);
   DevBuf<double2> o((size_t)nb * n3d);
   DevBuf<float4> bl;
-  launch_ae_states(t.view, proj_rows(d, kq, b0), d.proj.Ptot, kq, bloch_table(d, t, kq, bl), std::pow(d.vol, -0.5),
-                   g.p, n3d, nb, t.N, o.p);
+  with_bloch(d, t, kq, bl, [&](const BlochSlab &slab) {
+    launch_ae_states(t.view, proj_rows(d, kq, b0), d.proj.Ptot, kq, slab, std::pow(d.vol, -0.5), g.p, n3d, nb, t.N, o.p);
+  });
   o.download(reinterpret_cast<double2 *>(x), o.n);
   sync();
 }
@@ -2382,17 +2422,29 @@ static void ae_density(DevWF &d, AeTables &t, int kq, const std::vector<int> &ba
   DevBuf<float2> wd(std::max<size_t>(1, ws.size()));
   wd.upload(ws.data(), ws.size());
   DevBuf<float4> bl;
-  const float4 *bloch = bands.empty() ? nullptr : bloch_table(d, t, kq, bl);
-  // runs of consecutive bands in batches
-  for (size_t i = 0; i < bands.size();) {
+  // runs of consecutive bands, in batches that the free memory holds
+  const long long per_band = ncell * (long long)sizeof(float2) + rs_band_bytes(d, t, kq);
+  const size_t step = (size_t)scratch_count(std::min<size_t>(kAeBatch, std::max<size_t>(1, bands.size())), per_band,
+                                            std::numeric_limits<long long>::max());
+  auto run_end = [&](size_t i) {
     size_t j = i + 1;
-    while (j < bands.size() && bands[j] == bands[j - 1] + 1 && j - i < (size_t)kAeBatch) j++;
+    while (j < bands.size() && bands[j] == bands[j - 1] + 1 && j - i < step) j++;
+    return j;
+  };
+  size_t longest = 0;
+  for (size_t i = 0, j; i < bands.size(); i = j) {
+    j = run_end(i);
+    longest = std::max(longest, j - i);
+  }
+  if (g.n < longest * ncell) g.alloc(longest * ncell);
+  for (size_t i = 0, j; i < bands.size(); i = j) {
+    j = run_end(i);
     const int nb = (int)(j - i);
-    if (g.n < (size_t)nb * ncell) g.alloc((size_t)std::min<size_t>(kAeBatch, bands.size()) * ncell);
     rs_grids(d, t, kq, bands[i], nb, g.p, ncell);
-    launch_ae_density(t.view, proj_rows(d, kq, bands[i]), d.proj.Ptot, kq, bloch, std::pow(d.vol, -0.5), g.p, ncell,
-                      nb, t.N, wd.p + i, rho);
-    i = j;
+    with_bloch(d, t, kq, bl, [&](const BlochSlab &slab) {
+      launch_ae_density(t.view, proj_rows(d, kq, bands[i]), d.proj.Ptot, kq, slab, std::pow(d.vol, -0.5), g.p, ncell, nb,
+                        t.N, wd.p + i, rho);
+    });
   }
 }
 
@@ -3012,19 +3064,18 @@ static void ae_grid_rows(DevWF &d, AeTables &t, int kq, int b0, int nb, float2 *
   if (ld > n3d)
     PAWPY_CUDA(cudaMemset2DAsync(rows + n3d, sizeof(float2) * ld, 0, sizeof(float2) * (ld - n3d), nb, stream()));
   DevBuf<float4> bl;
-  const float4 *bloch = bloch_table(d, t, kq, bl);
-  // batches whose intermediate planes stay within about 1 GiB
-  const long long line = (long long)t.N[0] * t.N[1] * t.N[2] * (long long)sizeof(float2);
-  const int step = (int)std::max(1LL, (1LL << 30) / line);
+  const int step = scratch_count(nb, rs_band_bytes(d, t, kq), 1LL << 30);
   for (int b = 0; b < nb; b += step) {
     const int n = std::min(step, nb - b);
     rs_grids(d, t, kq, b0 + b, n, rows + (size_t)b * ld, ld);
-    launch_ae_store(t.view, proj_rows(d, kq, b0 + b), d.proj.Ptot, kq, bloch, std::pow(d.vol, -0.5),
-                    rows + (size_t)b * ld, ld, n, t.N);
+    with_bloch(d, t, kq, bl, [&](const BlochSlab &slab) {
+      launch_ae_store(t.view, proj_rows(d, kq, b0 + b), d.proj.Ptot, kq, slab, std::pow(d.vol, -0.5),
+                      rows + (size_t)b * ld, ld, n, t.N);
+    });
   }
 }
 
-// Memory for the grids of both sides of the real-space overlaps, in k-points at once.
+// The most memory that the grids of both sides of the real-space overlaps take, in k-points at once.
 constexpr long long kAeOverlapBytes = 8LL << 30;
 
 // <psi_R,bR,k|psi_S,bS,k> of the all-electron real-space wavefunctions on grid fftg for the
@@ -3045,7 +3096,7 @@ static void realspace_overlaps(pswf_t *wf_S, pswf_t *wf_R, const int *fftg, cons
   const int nk = S.nk, nbR = R.nband;
   const double scale = S.vol / (double)n3d;
   const long long per_k = (long long)(ns + nbR) * ld * (long long)sizeof(float2);
-  const int kb = (int)std::min<long long>(nk, std::max(1LL, kAeOverlapBytes / per_k));
+  const int kb = scratch_count(nk, per_k, kAeOverlapBytes);
   DevBuf<float2> gS((size_t)kb * ns * ld), gR((size_t)kb * nbR * ld), o((size_t)nk * ns * nbR);
   for (int k0 = 0; k0 < nk; k0 += kb) {
     const int n = std::min(kb, nk - k0);

@@ -347,16 +347,21 @@ void launch_rs_fft(const float2 *C, int Wpad, const RsPlan &pl, const int *N, co
 // (lengths rs_fft.cu has no split for)
 void launch_scatter_bands(const float2 *C, int Wpad, const int *gsorted, int W, int N1, int N2, int N3,
                           float2 *grid, int nb);
-// scale exp(2 pi i k.r) of every cell as (hi, lo) pairs of cosine and sine
-void launch_bloch_table(const int *N, const double *kfrac, double scale, float4 *out);
-// psi_b = scale exp(2 pi i k.r) grid_b + the sphere terms of the projector coefficients P[b][Pstride] of
-// k-point kq (bloch: the table, nullptr at Gamma): rho[cell] += sum_b w_b |psi_b|^2 (w_b = x + y); psi_b back
-// into the grids; psi_b as complex128 [b][cell]
-void launch_ae_density(const AeSpread &c, const float2 *P, int Pstride, int kq, const float4 *bloch, double scale,
+// Cells [x0, x0 + nx) of the first axis and their Bloch factors, from the slab's first cell (nullptr at Gamma).
+struct BlochSlab {
+  const float4 *p;
+  int x0, nx;
+};
+// scale exp(2 pi i k.r) of the slab's cells as (hi, lo) pairs of cosine and sine
+void launch_bloch_table(const int *N, const BlochSlab &slab, const double *kfrac, double scale, float4 *out);
+// On the slab's cells: psi_b = scale exp(2 pi i k.r) grid_b + the sphere terms of the projector coefficients
+// P[b][Pstride] of k-point kq: rho[cell] += sum_b w_b |psi_b|^2 (w_b = x + y); psi_b back into the grids; psi_b as
+// complex128 [b][cell]
+void launch_ae_density(const AeSpread &c, const float2 *P, int Pstride, int kq, const BlochSlab &slab, double scale,
                        float2 *grid, long long stride, int nb, const int *N, const float2 *w, double *rho);
-void launch_ae_store(const AeSpread &c, const float2 *P, int Pstride, int kq, const float4 *bloch, double scale,
+void launch_ae_store(const AeSpread &c, const float2 *P, int Pstride, int kq, const BlochSlab &slab, double scale,
                      float2 *grid, long long stride, int nb, const int *N);
-void launch_ae_states(const AeSpread &c, const float2 *P, int Pstride, int kq, const float4 *bloch, double scale,
+void launch_ae_states(const AeSpread &c, const float2 *P, int Pstride, int kq, const BlochSlab &slab, double scale,
                       float2 *grid, long long stride, int nb, const int *N, double2 *out);
 // x[i] *= exp(-2 pi i k.r_frac) on a host-layout double grid
 void launch_remove_phase(double2 *x, int N1, int N2, int N3, const double *kfrac);

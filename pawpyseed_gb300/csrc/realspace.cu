@@ -323,9 +323,9 @@ __global__ void k_ae_transpose(const float2 *__restrict__ P, int Pstride, int nb
 
 // (c, s) = scale exp(2 pi i k.(i/N1, j/N2, k/N3)) of every cell as pairs of FP32 (hi, lo), 48 bits:
 // (c hi, c lo, s hi, s lo); one CTA per row of the third axis
-__global__ void k_bloch_table(int N1, int N2, int N3, double kx, double ky, double kz, double scale,
+__global__ void k_bloch_table(int N1, int N2, int N3, int x0, double kx, double ky, double kz, double scale,
                               float4 *__restrict__ out) {
-  const int ij = blockIdx.x, i = ij / N2, j = ij % N2;
+  const int ij = blockIdx.x, i = x0 + ij / N2, j = ij % N2;
   const double base = kx * i / N1 + ky * j / N2;
   for (int k = threadIdx.x; k < N3; k += blockDim.x) {
     double a = base + kz * k / N3;
@@ -358,7 +358,8 @@ __device__ __forceinline__ float ds_rot(float x, float y, float ch, float cl, fl
 }
 
 // psi_b(cell) = scale exp(2 pi i k.r) u_b(cell) + sum over the cell's entries of
-//   phase sum_n val_n P_b,n, bands b < nb of the tiles of NB (blockIdx.y); one thread per cell.
+//   phase sum_n val_n P_b,n, bands b < nb of the tiles of NB (blockIdx.y); one thread per cell of the slab
+// [x0, x1) of the first axis (bloch: its factors).
 // MODE 0: rho[cell] += sum_b w_b |psi_b|^2; MODE 1: psi back into the grid; MODE 2: psi to out
 // (complex128).
 //
@@ -375,16 +376,16 @@ __device__ __forceinline__ float ds_rot(float x, float y, float ch, float cl, fl
 template <int NB, int MODE>
 __global__ void __launch_bounds__(128, NB == 16 ? 4 : 8)
     k_ae_apply(AeSpread c, const float4 *__restrict__ PT, int Pstride, int kq, const float4 *__restrict__ bloch,
-               float2 scale, float2 *__restrict__ grid, long long stride, int nb, int N1, int N2, int N3,
-               const float2 *__restrict__ w, double *__restrict__ rho, double2 *__restrict__ out) {
+               float2 scale, float2 *__restrict__ grid, long long stride, int nb, int x0, int x1, int N2, int N3,
+               int ncell, const float2 *__restrict__ w, double *__restrict__ rho, double2 *__restrict__ out) {
   constexpr int NP = NB / 2;  // band pairs
   // brick of the warp: z fastest
   const int bz = (N3 + 3) / 4, by = (N2 + 3) / 4;
   const int brick = blockIdx.x * (blockDim.x / 32) + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   const int z = brick % bz * 4 + (lane & 3), y = brick / bz % by * 4 + (lane >> 2 & 3),
-            x = brick / (bz * by) * 2 + (lane >> 4);
-  if (x >= N1 || y >= N2 || z >= N3) return;
-  const int cell = (x * N2 + y) * N3 + z, ncell = N1 * N2 * N3;
+            x = x0 + brick / (bz * by) * 2 + (lane >> 4);
+  if (x >= x1 || y >= N2 || z >= N3) return;
+  const int cell = (x * N2 + y) * N3 + z;
   const int b0 = blockIdx.y * NB;
   const float4 *pt = PT + (long long)blockIdx.y * Pstride * NP;
   const float2 *ph = c.phase + (long long)kq * c.npts;
@@ -428,7 +429,7 @@ __global__ void __launch_bounds__(128, NB == 16 ? 4 : 8)
     }
   }
   // (at Gamma the factor is the scale)
-  const float4 bl = bloch ? bloch[cell] : make_float4(scale.x, scale.y, 0.f, 0.f);
+  const float4 bl = bloch ? bloch[cell - x0 * N2 * N3] : make_float4(scale.x, scale.y, 0.f, 0.f);
   float2 acc = make_float2(0.f, 0.f);
 #pragma unroll
   for (int i = 0; i < NB; i++) {
@@ -456,17 +457,17 @@ __global__ void __launch_bounds__(128, NB == 16 ? 4 : 8)
   if constexpr (MODE == 0) rho[cell] += (double)acc.x + (double)acc.y;
 }
 
-void launch_bloch_table(const int *N, const double *kfrac, double scale, float4 *out) {
-  PAWPY_LAUNCH("ae_apply", k_bloch_table<<<N[0] * N[1], 128, 0, stream()>>>(N[0], N[1], N[2], kfrac[0], kfrac[1],
-                                                                          kfrac[2], scale, out));
+void launch_bloch_table(const int *N, const BlochSlab &slab, const double *kfrac, double scale, float4 *out) {
+  PAWPY_LAUNCH("ae_apply", k_bloch_table<<<slab.nx * N[1], 128, 0, stream()>>>(N[0], N[1], N[2], slab.x0, kfrac[0],
+                                                                             kfrac[1], kfrac[2], scale, out));
 }
 
 namespace {
 
 template <int MODE>
-void ae_apply(const AeSpread &c, const float2 *P, int Pstride, int kq, const float4 *bloch, double scale, float2 *grid,
+void ae_apply(const AeSpread &c, const float2 *P, int Pstride, int kq, const BlochSlab &slab, double scale, float2 *grid,
               long long stride, int nb, const int *N, const float2 *w, double *rho, double2 *out) {
-  if (nb <= 0) return;
+  if (nb <= 0 || slab.nx <= 0) return;
   // 16 bands per thread; narrower for a few bands
   const int NB = nb <= 2 ? 2 : nb <= 4 ? 4 : 16, tiles = ceil_div(nb, NB);
   DevBuf<float4> PT((size_t)tiles * std::max(1, Pstride) * NB / 2);
@@ -475,31 +476,32 @@ void ae_apply(const AeSpread &c, const float2 *P, int Pstride, int kq, const flo
                                  P, Pstride, nb, NB, PT.p));
   const float hi = (float)scale;
   const float2 sc = make_float2(hi, (float)(scale - hi));
-  const long long bricks = (long long)ceil_div(N[0], 2) * ceil_div(N[1], 4) * ceil_div(N[2], 4);
+  const long long bricks = (long long)ceil_div(slab.nx, 2) * ceil_div(N[1], 4) * ceil_div(N[2], 4);
   auto fn = NB == 2 ? k_ae_apply<2, MODE> : NB == 4 ? k_ae_apply<4, MODE> : k_ae_apply<16, MODE>;
   // the density sums over the tiles: one launch per tile (each adds to rho)
   const int per = MODE == 0 ? 1 : tiles;
   for (int t = 0; t < tiles; t += per) {
     const int b = t * NB, n = std::min(nb - b, per * NB);
     PAWPY_LAUNCH("ae_apply", fn<<<dim3(ceil_div(bricks, 4), per), 128, 0, stream()>>>(
-                                 c, PT.p + (size_t)t * Pstride * NB / 2, Pstride, kq, bloch, sc, grid + b * stride,
-                                 stride, n, N[0], N[1], N[2], w ? w + b : nullptr, rho, out));
+                                 c, PT.p + (size_t)t * Pstride * NB / 2, Pstride, kq, slab.p, sc, grid + b * stride,
+                                 stride, n, slab.x0, slab.x0 + slab.nx, N[1], N[2], N[0] * N[1] * N[2],
+                                 w ? w + b : nullptr, rho, out));
   }
 }
 
 }  // namespace
 
-void launch_ae_density(const AeSpread &c, const float2 *P, int Pstride, int kq, const float4 *bloch, double scale,
+void launch_ae_density(const AeSpread &c, const float2 *P, int Pstride, int kq, const BlochSlab &slab, double scale,
                        float2 *grid, long long stride, int nb, const int *N, const float2 *w, double *rho) {
-  ae_apply<0>(c, P, Pstride, kq, bloch, scale, grid, stride, nb, N, w, rho, nullptr);
+  ae_apply<0>(c, P, Pstride, kq, slab, scale, grid, stride, nb, N, w, rho, nullptr);
 }
-void launch_ae_store(const AeSpread &c, const float2 *P, int Pstride, int kq, const float4 *bloch, double scale,
+void launch_ae_store(const AeSpread &c, const float2 *P, int Pstride, int kq, const BlochSlab &slab, double scale,
                      float2 *grid, long long stride, int nb, const int *N) {
-  ae_apply<1>(c, P, Pstride, kq, bloch, scale, grid, stride, nb, N, nullptr, nullptr, nullptr);
+  ae_apply<1>(c, P, Pstride, kq, slab, scale, grid, stride, nb, N, nullptr, nullptr, nullptr);
 }
-void launch_ae_states(const AeSpread &c, const float2 *P, int Pstride, int kq, const float4 *bloch, double scale,
+void launch_ae_states(const AeSpread &c, const float2 *P, int Pstride, int kq, const BlochSlab &slab, double scale,
                       float2 *grid, long long stride, int nb, const int *N, double2 *out) {
-  ae_apply<2>(c, P, Pstride, kq, bloch, scale, grid, stride, nb, N, nullptr, nullptr, out);
+  ae_apply<2>(c, P, Pstride, kq, slab, scale, grid, stride, nb, N, nullptr, nullptr, out);
 }
 
 // x[i] *= exp(-2 pi i k.(i/N1, j/N2, k/N3)) in double precision (remove_phase)

@@ -72,3 +72,69 @@ def test_realspace_projections_of_more_than_a_thousand_k_points():
         S = np.array([wf.get_state_realspace(b, k, 0, dim=(32, 32, 32)).ravel() for b in range(2)])
         R = np.array([basis.get_state_realspace(b, k, 0, dim=(32, 32, 32)).ravel() for b in range(3)])
         assert np.abs(out[:, k::1100] - S @ R.conj().T * vol / n3).max() <= 1e-5
+
+
+def test_scratch_of_the_real_space_functions_follows_the_free_memory():
+    pieces = rule("_ZN5pawpy14scratch_piecesExxxx", C.c_int, C.c_longlong, C.c_longlong, C.c_longlong, C.c_longlong)
+    MB, many = 1 << 20, 1 << 62
+    # 16 band grids of 216 MB: all on a free device, four of them in 4 GB, one where even that does not fit
+    assert pieces(16, 216 * MB, many, 270 * GB) == 16
+    assert pieces(16, 216 * MB, many, 4 * GB) == 4
+    assert pieces(16, 216 * MB, many, 1 * GB) == 1
+    assert pieces(16, 1100 * MB, many, 2 * GB) == 1
+    # k-points of 500 MB: at most 8 GB of them
+    assert pieces(100, 500 * MB, 8 * GB, 270 * GB) == 16
+    # little scratch is taken whatever is free
+    assert pieces(16, 16 * MB, many, 0) == 16
+
+
+DENSITY = """
+import numpy as np, torch
+from test_gpu_fft_grouped import wavefunction
+from pawpyseed_gb300 import _lib, synth, vaspio
+from pawpyseed_gb300.wavefunction import Wavefunction
+st, _ = synth.structures(0)
+cr = vaspio.CoreRegion(synth.potcar_text(["A"]))
+w = dict(encut=30.0, kpts=np.array([[0.1, 0.2, 0.3]]), nband=32, nspin=1, dim=(16, 16, 16))
+data = synth.wavefunction_data(st, w, 3)
+data["occs"] = np.asarray([[[float(b % 2 == 0) for b in range(32)]]]).reshape(np.asarray(data["occs"]).shape)
+wf = Wavefunction.from_arrays(st, cr, (16, 16, 16), data)
+wf.get_realspace_density(dim=(18, 18, 18))
+wf.get_state_realspace(0, 0, 0, dim=(216, 216, 216))  # the sphere tables of the grid
+_lib.lib().pawpy_gpu_synchronize()
+free = torch.cuda.mem_get_info()[0]
+wf.get_realspace_density(dim=(216, 216, 216))
+_lib.lib().pawpy_gpu_synchronize()
+print((free - torch.cuda.mem_get_info()[0]) // (8 * 216**3))
+"""
+
+
+@pytest.mark.gpu
+def test_density_of_separate_bands_holds_one_grid_at_a_time():
+    """16 occupied bands, none beside another: the grids the call adds to the pool (one band's and its density
+    fit in what the state before it left there) are fewer than a few, not 16."""
+    import os
+    import subprocess
+    import sys
+
+    from conftest import ROOT
+
+    env = dict(os.environ, PYTHONPATH=os.pathsep.join([ROOT, os.path.join(ROOT, "tests")]))
+    r = subprocess.run([sys.executable, "-c", DENSITY], capture_output=True, text=True, env=env, cwd=ROOT)
+    assert r.returncode == 0, r.stderr
+    assert int(r.stdout.split()[-1]) <= 4
+
+
+@pytest.mark.gpu
+def test_state_on_a_grid_whose_bloch_factors_are_tabulated_in_slabs():
+    """270 x 256 x 252 points (a table of 279 MB) against every other point's grid, where it is built whole: the
+    same values at the same points, 1e-5 of the largest as the other states."""
+    from test_gpu_fft_grouped import wavefunction
+
+    wf, _ = wavefunction((16, 16, 16), 60.0)
+    fine = wf.get_state_realspace(3, 1, 0, dim=(270, 256, 252))[::2, ::2, ::2]
+    coarse = wf.get_state_realspace(3, 1, 0, dim=(135, 128, 126))
+    assert np.abs(fine - coarse).max() <= 1e-5 * np.abs(coarse).max()
+    rf = wf.get_realspace_density(dim=(270, 256, 252))[::2, ::2, ::2]
+    rc = wf.get_realspace_density(dim=(135, 128, 126))
+    assert np.abs(rf - rc).max() <= 1e-5 * np.abs(rc).max()
