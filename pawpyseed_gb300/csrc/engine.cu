@@ -2340,9 +2340,11 @@ static bool rs_sparse(DevWF &d, AeTables &t, int kq) {
   return v;
 }
 
-// scratch of rs_grids per band, at most
-static long long rs_band_bytes(DevWF &d, AeTables &t, int kq) {
-  return rs_sparse(d, t, kq) ? 2LL * std::max(1, d.kp[kq].n1) * t.N[1] * t.N[2] * (long long)sizeof(float2) : 0;
+// scratch of rs_grids per band, at most (rows past the grid, stride > cells, need a copy in the whole-grid form)
+static long long rs_band_bytes(DevWF &d, AeTables &t, int kq, long long stride) {
+  const long long plane = (long long)t.N[1] * t.N[2], n3d = plane * t.N[0];
+  const long long n = rs_sparse(d, t, kq) ? 2 * std::max(1, d.kp[kq].n1) * plane : stride == n3d ? 0 : n3d;
+  return n * (long long)sizeof(float2);
 }
 
 // sum_G C_G exp(i G.r) of bands [b0, b0 + nb) of k-point kq on the grid of t, grid[b stride + cell].
@@ -2361,11 +2363,14 @@ static void rs_grids(DevWF &d, AeTables &t, int kq, int b0, int nb, float2 *grid
     q.gs_d.alloc(std::max<size_t>(3, q.gsorted.size()));
     q.gs_d.upload(q.gsorted.data(), q.gsorted.size());
   }
-  for (int b = 0; b < nb; b++) {
-    float2 *g = grid + b * stride;
-    launch_scatter_bands(C + (size_t)b * q.Wpad, q.Wpad, q.gs_d.p, q.W, N[0], N[1], N[2], g, 1);
-    for (int a = 2; a >= 0; a--) launch_fft_axis(g, 1, N[0], N[1], N[2], a, t.r[a], t.tw[a].p);
-  }
+  const long long n3d = (long long)N[0] * N[1] * N[2];
+  DevBuf<float2> tmp(stride == n3d ? 0 : (size_t)nb * n3d);
+  float2 *g = stride == n3d ? grid : tmp.p;
+  launch_scatter_bands(C, q.Wpad, q.gs_d.p, q.W, N[0], N[1], N[2], g, nb);
+  for (int a = 2; a >= 0; a--) launch_fft_axis(g, nb, N[0], N[1], N[2], a, t.r[a], t.tw[a].p);
+  if (tmp.n)
+    PAWPY_CUDA(cudaMemcpy2DAsync(grid, sizeof(float2) * stride, g, sizeof(float2) * n3d, sizeof(float2) * n3d, nb,
+                                 cudaMemcpyDeviceToDevice, stream()));
 }
 
 // rows of the projector coefficients of bands from b0 of k-point kq
@@ -2423,7 +2428,7 @@ static void ae_density(DevWF &d, AeTables &t, int kq, const std::vector<int> &ba
   wd.upload(ws.data(), ws.size());
   DevBuf<float4> bl;
   // runs of consecutive bands, in batches that the free memory holds
-  const long long per_band = ncell * (long long)sizeof(float2) + rs_band_bytes(d, t, kq);
+  const long long per_band = ncell * (long long)sizeof(float2) + rs_band_bytes(d, t, kq, ncell);
   const size_t step = (size_t)scratch_count(std::min<size_t>(kAeBatch, std::max<size_t>(1, bands.size())), per_band,
                                             std::numeric_limits<long long>::max());
   auto run_end = [&](size_t i) {
@@ -3064,7 +3069,7 @@ static void ae_grid_rows(DevWF &d, AeTables &t, int kq, int b0, int nb, float2 *
   if (ld > n3d)
     PAWPY_CUDA(cudaMemset2DAsync(rows + n3d, sizeof(float2) * ld, 0, sizeof(float2) * (ld - n3d), nb, stream()));
   DevBuf<float4> bl;
-  const int step = scratch_count(nb, rs_band_bytes(d, t, kq), 1LL << 30);
+  const int step = scratch_count(nb, rs_band_bytes(d, t, kq, ld), 1LL << 30);
   for (int b = 0; b < nb; b += step) {
     const int n = std::min(step, nb - b);
     rs_grids(d, t, kq, b0 + b, n, rows + (size_t)b * ld, ld);
