@@ -2127,16 +2127,23 @@ static void do_overlap_setup_recip(pswf_t *wf_R, pswf_t *wf_S, const int *labels
 // ============================================================= all-electron real-space wavefunctions
 
 // How many of `want` equal pieces of scratch (band grids, k-points) a real-space call holds at once, at least one:
-// what a quarter of the free device memory and `cap` hold, or 256 MiB if that is more.
-constexpr long long kScratchBytes = 256LL << 20;
+// what a quarter of the free device memory and `cap` hold, or 1 GiB if that is more.
+constexpr long long kScratchBytes = 1LL << 30;
 int scratch_pieces(long long want, long long bytes_each, long long cap, long long free_bytes) {
   const long long budget = std::max(kScratchBytes, std::min(cap, free_bytes / 4));
   return (int)std::max(1LL, std::min(want, budget / std::max(1LL, bytes_each)));
 }
-// (the free memory is asked for where the pieces need more than that)
-static int scratch_count(long long want, long long bytes_each, long long cap) {
-  return scratch_pieces(want, bytes_each, cap, want * bytes_each <= kScratchBytes ? 0 : free_device_bytes());
-}
+// The same within one call of the library: the free memory is asked for once, and only where the pieces need more than
+// 1 GiB (asking takes 0.2 ms; per k-point it took a quarter of the density of 64 atoms on 120^3).
+struct ScratchBudget {
+  int count(long long want, long long bytes_each, long long cap) {
+    if (want * bytes_each > kScratchBytes && cap > kScratchBytes && free_ < 0) free_ = free_device_bytes();
+    return scratch_pieces(want, bytes_each, cap, std::max(0LL, free_));
+  }
+
+ private:
+  long long free_ = -1;
+};
 
 // The real-space sphere tables of d's sites on grid N (built once per grid and site list).
 static AeTables &ae_tables(DevWF &d, const int *N, const int *labels, const double *coords) {
@@ -2379,13 +2386,14 @@ static const float2 *proj_rows(DevWF &d, int kq, int b0) {
 }
 
 // The Bloch factors of k-point kq on the grid of t (scale included): f(slab) for the whole grid, or for one slab
-// of the first axis after another where the grid's table (16 bytes per cell) would be larger than kScratchBytes. buf keeps
+// of the first axis after another where the grid's table (16 bytes per cell) would be larger than kBlochBytes. buf keeps
 // the whole grid's for the k-point's other calls.
+constexpr long long kBlochBytes = 256LL << 20;
 template <typename F>
 static void with_bloch(DevWF &d, AeTables &t, int kq, DevBuf<float4> &buf, F &&f) {
   const int *N = t.N;
   const long long plane = (long long)N[1] * N[2];
-  const int nx = (int)std::max(1LL, std::min<long long>(N[0], kScratchBytes / (plane * (long long)sizeof(float4))));
+  const int nx = (int)std::max(1LL, std::min<long long>(N[0], kBlochBytes / (plane * (long long)sizeof(float4))));
   if (kpoint_is_gamma(d.kp[kq])) {
     f(BlochSlab{nullptr, 0, N[0]});
     return;
@@ -2420,7 +2428,7 @@ constexpr int kAeBatch = 16;
 
 // rho += sum of w |psi|^2 over the given bands of k-point kq (density.c:158-204).
 static void ae_density(DevWF &d, AeTables &t, int kq, const std::vector<int> &bands, const std::vector<double> &w,
-                       DevBuf<float2> &g, double *rho) {
+                       ScratchBudget &mem, DevBuf<float2> &g, double *rho) {
   const int ncell = t.N[0] * t.N[1] * t.N[2];
   std::vector<float2> ws;
   for (double v : w) ws.push_back(make_float2((float)v, (float)(v - (float)v)));
@@ -2429,8 +2437,8 @@ static void ae_density(DevWF &d, AeTables &t, int kq, const std::vector<int> &ba
   DevBuf<float4> bl;
   // runs of consecutive bands, in batches that the free memory holds
   const long long per_band = ncell * (long long)sizeof(float2) + rs_band_bytes(d, t, kq, ncell);
-  const size_t step = (size_t)scratch_count(std::min<size_t>(kAeBatch, std::max<size_t>(1, bands.size())), per_band,
-                                            std::numeric_limits<long long>::max());
+  const size_t step = (size_t)mem.count(std::min<size_t>(kAeBatch, std::max<size_t>(1, bands.size())), per_band,
+                                        std::numeric_limits<long long>::max());
   auto run_end = [&](size_t i) {
     size_t j = i + 1;
     while (j < bands.size() && bands[j] == bands[j - 1] + 1 && j - i < step) j++;
@@ -3069,7 +3077,7 @@ static void ae_grid_rows(DevWF &d, AeTables &t, int kq, int b0, int nb, float2 *
   if (ld > n3d)
     PAWPY_CUDA(cudaMemset2DAsync(rows + n3d, sizeof(float2) * ld, 0, sizeof(float2) * (ld - n3d), nb, stream()));
   DevBuf<float4> bl;
-  const int step = scratch_count(nb, rs_band_bytes(d, t, kq, ld), 1LL << 30);
+  const int step = scratch_pieces(nb, rs_band_bytes(d, t, kq, ld), kScratchBytes, 0);
   for (int b = 0; b < nb; b += step) {
     const int n = std::min(step, nb - b);
     rs_grids(d, t, kq, b0 + b, n, rows + (size_t)b * ld, ld);
@@ -3101,7 +3109,7 @@ static void realspace_overlaps(pswf_t *wf_S, pswf_t *wf_R, const int *fftg, cons
   const int nk = S.nk, nbR = R.nband;
   const double scale = S.vol / (double)n3d;
   const long long per_k = (long long)(ns + nbR) * ld * (long long)sizeof(float2);
-  const int kb = scratch_count(nk, per_k, kAeOverlapBytes);
+  const int kb = ScratchBudget().count(nk, per_k, kAeOverlapBytes);
   DevBuf<float2> gS((size_t)kb * ns * ld), gR((size_t)kb * nbR * ld), o((size_t)nk * ns * nbR);
   for (int k0 = 0; k0 < nk; k0 += kb) {
     const int n = std::min(kb, nk - k0);
@@ -3158,10 +3166,11 @@ void ae_state_density(double *P, int BAND_NUM, int KPOINT_NUM, pswf_t *wf, int *
   AeTables &t = ae_tables(d, fftg, labels, coords);
   const long long n3d = (long long)fftg[0] * fftg[1] * fftg[2];
   ensure_projections(d);
+  ScratchBudget mem;
   DevBuf<float2> g;
   DevBuf<double> rho(n3d);
   rho.upload(P, n3d);
-  ae_density(d, t, KPOINT_NUM, {BAND_NUM}, {1.0}, g, rho.p);
+  ae_density(d, t, KPOINT_NUM, {BAND_NUM}, {1.0}, mem, g, rho.p);
   rho.download(P, n3d);
   sync();
   PAWPY_API_END()
@@ -3176,6 +3185,7 @@ void ae_chg_density(double *P, pswf_t *wf, int *fftg, int *labels, double *coord
   AeTables &t = ae_tables(d, fftg, labels, coords);
   const long long n3d = (long long)fftg[0] * fftg[1] * fftg[2];
   ensure_projections(d);
+  ScratchBudget mem;
   DevBuf<float2> g;
   DevBuf<double> rho(n3d);
   rho.upload(P, n3d);
@@ -3191,7 +3201,7 @@ void ae_chg_density(double *P, pswf_t *wf, int *fftg, int *labels, double *coord
         wk.push_back(wf->kpts[k]->weight * bd->occ * spin_mult);
       }
     }
-    ae_density(d, t, k, occ, wk, g, rho.p);
+    ae_density(d, t, k, occ, wk, mem, g, rho.p);
   }
   rho.download(P, n3d);
   sync();
@@ -3224,6 +3234,7 @@ void ncl_ae_chg_density(double *P, pswf_t *wf, int *fftg, int *labels, double *c
   AeTables &t = ae_tables(d, fftg, labels, coords);
   const long long n3d = (long long)fftg[0] * fftg[1] * fftg[2];
   ensure_projections(d);
+  ScratchBudget mem;
   DevBuf<float2> g;
   DevBuf<double> rho(n3d);
   rho.upload(P, n3d);
@@ -3239,7 +3250,7 @@ void ncl_ae_chg_density(double *P, pswf_t *wf, int *fftg, int *labels, double *c
           wk.push_back(wf->kpts[k]->weight * bd->occ);
         }
     }
-    ae_density(d, t, k, occ, wk, g, rho.p);
+    ae_density(d, t, k, occ, wk, mem, g, rho.p);
   }
   rho.download(P, n3d);
   sync();

@@ -359,7 +359,7 @@ __device__ __forceinline__ float ds_rot(float x, float y, float ch, float cl, fl
 
 // psi_b(cell) = scale exp(2 pi i k.r) u_b(cell) + sum over the cell's entries of
 //   phase sum_n val_n P_b,n, bands b < nb of the tiles of NB (blockIdx.y); one thread per cell of the slab
-// [x0, x1) of the first axis (bloch: its factors).
+// [x0, x1) of the first axis (bloch: the factors by cell).
 // MODE 0: rho[cell] += sum_b w_b |psi_b|^2; MODE 1: psi back into the grid; MODE 2: psi to out
 // (complex128).
 //
@@ -429,7 +429,7 @@ __global__ void __launch_bounds__(128, NB == 16 ? 4 : 8)
     }
   }
   // (at Gamma the factor is the scale)
-  const float4 bl = bloch ? bloch[cell - x0 * N2 * N3] : make_float4(scale.x, scale.y, 0.f, 0.f);
+  const float4 bl = bloch ? bloch[cell] : make_float4(scale.x, scale.y, 0.f, 0.f);
   float2 acc = make_float2(0.f, 0.f);
 #pragma unroll
   for (int i = 0; i < NB; i++) {
@@ -478,12 +478,13 @@ void ae_apply(const AeSpread &c, const float2 *P, int Pstride, int kq, const Blo
   const float2 sc = make_float2(hi, (float)(scale - hi));
   const long long bricks = (long long)ceil_div(slab.nx, 2) * ceil_div(N[1], 4) * ceil_div(N[2], 4);
   auto fn = NB == 2 ? k_ae_apply<2, MODE> : NB == 4 ? k_ae_apply<4, MODE> : k_ae_apply<16, MODE>;
+  const float4 *bloch = slab.p ? slab.p - (long long)slab.x0 * N[1] * N[2] : nullptr;
   // the density sums over the tiles: one launch per tile (each adds to rho)
   const int per = MODE == 0 ? 1 : tiles;
   for (int t = 0; t < tiles; t += per) {
     const int b = t * NB, n = std::min(nb - b, per * NB);
     PAWPY_LAUNCH("ae_apply", fn<<<dim3(ceil_div(bricks, 4), per), 128, 0, stream()>>>(
-                                 c, PT.p + (size_t)t * Pstride * NB / 2, Pstride, kq, slab.p, sc, grid + b * stride,
+                                 c, PT.p + (size_t)t * Pstride * NB / 2, Pstride, kq, bloch, sc, grid + b * stride,
                                  stride, n, slab.x0, slab.x0 + slab.nx, N[1], N[2], N[0] * N[1] * N[2],
                                  w ? w + b : nullptr, rho, out));
   }

@@ -77,15 +77,15 @@ def test_realspace_projections_of_more_than_a_thousand_k_points():
 def test_scratch_of_the_real_space_functions_follows_the_free_memory():
     pieces = rule("_ZN5pawpy14scratch_piecesExxxx", C.c_int, C.c_longlong, C.c_longlong, C.c_longlong, C.c_longlong)
     MB, many = 1 << 20, 1 << 62
-    # 16 band grids of 216 MB: all on a free device, four of them in 4 GB, one where even that does not fit
+    # 16 band grids of 216 MB: all on a free device, nine of them in 8 GB, four (1 GiB) where little is free
     assert pieces(16, 216 * MB, many, 270 * GB) == 16
-    assert pieces(16, 216 * MB, many, 4 * GB) == 4
-    assert pieces(16, 216 * MB, many, 1 * GB) == 1
+    assert pieces(16, 216 * MB, many, 8 * GB) == 9
+    assert pieces(16, 216 * MB, many, 1 * GB) == 4
     assert pieces(16, 1100 * MB, many, 2 * GB) == 1
     # k-points of 500 MB: at most 8 GB of them
     assert pieces(100, 500 * MB, 8 * GB, 270 * GB) == 16
     # little scratch is taken whatever is free
-    assert pieces(16, 16 * MB, many, 0) == 16
+    assert pieces(16, 64 * MB, many, 0) == 16
 
 
 DENSITY = """
