@@ -348,14 +348,46 @@ __device__ __forceinline__ void ds_add(float2 &a, float hi, float lo) {
 }
 
 // x c - y s with c and s as (hi, lo) pairs, rounded once to FP32 (but for about one value in 2^20
-// that lies within 2^-44 of a rounding boundary)
+// that lies within 2^-44 of a rounding boundary); infinities and NaN as in the plain product, whose corrections
+// are then not finite
 __device__ __forceinline__ float ds_rot(float x, float y, float ch, float cl, float sh, float sl) {
   const float p = __fmul_rn(x, ch), q = __fmul_rn(y, sh);
   const float pe = __fmaf_rn(x, cl, __fmaf_rn(x, ch, -p)), qe = __fmaf_rn(y, sl, __fmaf_rn(y, sh, -q));
   const float d = __fsub_rn(p, q), v = __fsub_rn(d, p);
   const float e = __fsub_rn(__fsub_rn(p, __fsub_rn(d, v)), __fadd_rn(q, v));
-  return __fadd_rn(d, __fadd_rn(e, __fsub_rn(pe, qe)));
+  const float r = __fadd_rn(d, __fadd_rn(e, __fsub_rn(pe, qe)));
+  return fabsf(r) < INFINITY ? r : d;
 }
+
+// psi of the band at place i of its tile, as k_ae_apply evaluates it (pt: the tile's coefficients)
+__device__ __forceinline__ float2 ae_value(const AeSpread &c, const float4 *__restrict__ pt, int NP, int i,
+                                           const float2 *__restrict__ ph, int cell, float2 u, float4 bl) {
+  float ar = 0.f, ai = 0.f;
+  const int e1 = c.first[cell + 1];
+  for (int e = c.first[cell]; e < e1; e++) {
+    const int2 en = c.ent[e];
+    const AeSite si = c.sites[en.y];
+    const float2 *v = c.val + si.val + (long long)(en.x - si.pt) * ae_stride(si.total);
+    const float4 *pp = pt + (long long)si.pcol * NP + i / 2;
+    float yr = 0.f, yi = 0.f;
+#pragma unroll 1
+    for (int q = 0; q < si.total; q++) {
+      const float4 a = pp[q * NP];
+      const float re = i & 1 ? a.y : a.x, im = i & 1 ? a.w : a.z;
+      yr = __fadd_rn(yr, __fmaf_rn(re, v[q].x, __fmul_rn(im, -v[q].y)));
+      yi = __fadd_rn(yi, __fmaf_rn(re, v[q].y, __fmul_rn(im, v[q].x)));
+    }
+    const float2 f = ph[en.x];
+    ar = __fadd_rn(ar, __fmaf_rn(yr, f.x, __fmul_rn(yi, -f.y)));
+    ai = __fadd_rn(ai, __fmaf_rn(yr, f.y, __fmul_rn(yi, f.x)));
+  }
+  return make_float2(__fadd_rn(ds_rot(u.x, u.y, bl.x, bl.y, bl.z, bl.w), ar),
+                     __fadd_rn(ds_rot(u.y, -u.x, bl.x, bl.y, bl.z, bl.w), ai));
+}
+
+// The range in which squares and their products with the weights keep both halves of a double-single value:
+// the low half of 2^-90 is a multiple of 2^-138 (denormals end at 2^-149), and 16 bands of 2^100 do not overflow.
+constexpr float kDsMin = 0x1p-90f, kDsMax = 0x1p100f;
 
 // psi_b(cell) = scale exp(2 pi i k.r) u_b(cell) + sum over the cell's entries of
 //   phase sum_n val_n P_b,n, bands b < nb of the tiles of NB (blockIdx.y); one thread per cell of the slab
@@ -372,7 +404,7 @@ __device__ __forceinline__ float ds_rot(float x, float y, float ch, float cl, fl
 // FP64 runs at two operations per clock and SM here: the Bloch factor (once FP64 sine, cosine and
 // product per band and cell, 20 ms of that workload) is a table of double-single factors, applied in
 // double-single FP32; densities are summed in double-single over the tile's bands, then in FP64,
-// within 1e-13 of the FP64 sum.
+// within 1e-13 of the FP64 sum (cells whose squares FP32 pairs do not hold: in FP64).
 template <int NB, int MODE>
 __global__ void __launch_bounds__(128, NB == 16 ? 4 : 8)
     k_ae_apply(AeSpread c, const float4 *__restrict__ PT, int Pstride, int kq, const float4 *__restrict__ bloch,
@@ -431,6 +463,7 @@ __global__ void __launch_bounds__(128, NB == 16 ? 4 : 8)
   // (at Gamma the factor is the scale)
   const float4 bl = bloch ? bloch[cell] : make_float4(scale.x, scale.y, 0.f, 0.f);
   float2 acc = make_float2(0.f, 0.f);
+  float least = kDsMax, most = kDsMin;
 #pragma unroll
   for (int i = 0; i < NB; i++) {
     if (b0 + i >= nb) break;
@@ -448,13 +481,28 @@ __global__ void __launch_bounds__(128, NB == 16 ? 4 : 8)
       const float m = __fmul_rn(wb.x, t.x);
       const float me = __fadd_rn(__fmaf_rn(wb.x, t.x, -m), __fadd_rn(__fmul_rn(wb.x, t.y), __fmul_rn(wb.y, t.x)));
       ds_add(acc, m, me);
+      least = fminf(least, fminf(t.x, m));
+      most = fmaxf(most, fmaxf(t.x, m));
     } else if constexpr (MODE == 1) {
       *g = psi;
     } else {
       out[(long long)(b0 + i) * ncell + cell] = make_double2(psi.x, psi.y);
     }
   }
-  if constexpr (MODE == 0) rho[cell] += (double)acc.x + (double)acc.y;
+  if constexpr (MODE == 0) {
+    if (least >= kDsMin && most <= kDsMax) {
+      rho[cell] += (double)acc.x + (double)acc.y;
+      return;
+    }
+    // a square that FP32 pairs do not hold (or an exact zero): the cell's sum again, in FP64
+    double s = rho[cell];
+#pragma unroll 1
+    for (int i = 0; i < NB && b0 + i < nb; i++) {
+      const float2 psi = ae_value(c, pt, NP, i, ph, cell, grid[(b0 + i) * stride + cell], bl);
+      s += ((double)w[b0 + i].x + w[b0 + i].y) * ((double)psi.x * psi.x + (double)psi.y * psi.y);
+    }
+    rho[cell] = s;
+  }
 }
 
 void launch_bloch_table(const int *N, const BlochSlab &slab, const double *kfrac, double scale, float4 *out) {
