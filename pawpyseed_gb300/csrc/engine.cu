@@ -128,7 +128,7 @@ struct DevKpt {
   std::vector<int> invperm;  // original plane-wave index -> sorted position
   std::vector<int> gsorted;  // [W][3] in sorted order
   DevBuf<int> perm_d, plane_start, plane_off;
-  DevBuf<unsigned short> plane_pos;  // coefficient positions in the tile of fft_band.cu's first pass
+  DevBuf<unsigned short> plane_pos;  // coefficient positions in the tile of the grouped first pass (fft_band.cuh)
   DevBuf<int> inv_d;  // invperm on the device (host-read upload)
   DevBuf<int> gs_d;   // gsorted on the device (real-space wavefunctions)
   int off_N2 = 0, off_N3 = 0;
@@ -648,7 +648,8 @@ static bool choose_form(PlaneGeom &g) {
 
 // Plane lists of one k-point for the plane FFT: start[p] = first sorted
 // coefficient of g1 plane p, off[t] = cell j * N3 + k of coefficient t within its
-// plane, pos[t] its position in the grouped form's tile, and the occupied ranges of the other two axes.
+// plane, and the occupied ranges of the other two axes; pos[t], its position in the grouped form's tile, where
+// that form transforms the k-point.
 struct PlaneLists {
   std::vector<int> start, off;
   std::vector<unsigned short> pos;
@@ -663,17 +664,26 @@ static void plane_lists(const DevWF &d, const DevKpt &q, PlaneLists &pl) {
   int lo2 = 1 << 30, hi2 = -(1 << 30), lo3 = 1 << 30, hi3 = -(1 << 30);
   for (int t = 0; t < q.W; t++) {
     const int g2 = q.gsorted[3 * t + 1], g3 = q.gsorted[3 * t + 2];
+    pl.start[q.gsorted[3 * t] - q.g1min + 1]++;
     lo2 = std::min(lo2, g2);
     hi2 = std::max(hi2, g2);
     lo3 = std::min(lo3, g3);
     hi3 = std::max(hi3, g3);
   }
-  pl.pos.resize(q.W);
+  pl.g2min = q.W ? lo2 : 0;
+  pl.n2 = q.W ? hi2 - lo2 + 1 : 0;
+  pl.g3min = q.W ? lo3 : 0;
+  pl.n3 = q.W ? hi3 - lo3 + 1 : 0;
+  for (int p = 0; p < q.n1; p++) pl.maxcnt = std::max(pl.maxcnt, pl.start[p + 1]);
+  for (int p = 0; p < q.n1; p++) pl.start[p + 1] += pl.start[p];
+  PlaneGeom g{d.N[0], N2, N3, q.g1min, q.n1, pl.g2min, pl.n2, pl.g3min, pl.n3, pl.maxcnt};
+  const bool grouped = choose_form(g) && g.grouped;
+  const int ld = fft_band_tile_ld(N3);
+  if (grouped) pl.pos.resize(q.W);
   // indices inside (-N, N) wrap with one compare; others take the modulus
   const bool near = q.W == 0 || (lo2 > -N2 && hi2 < N2 && lo3 > -N3 && hi3 < N3);
   for (int t = 0; t < q.W; t++) {
-    const int g1 = q.gsorted[3 * t], g2 = q.gsorted[3 * t + 1], g3 = q.gsorted[3 * t + 2];
-    pl.start[g1 - q.g1min + 1]++;
+    const int g2 = q.gsorted[3 * t + 1], g3 = q.gsorted[3 * t + 2];
     int j, kk;
     if (near) {
       j = g2 < 0 ? g2 + N2 : g2;
@@ -683,16 +693,17 @@ static void plane_lists(const DevWF &d, const DevKpt &q, PlaneLists &pl) {
       kk = ((g3 % N3) + N3) % N3;
     }
     pl.off[t] = j * N3 + kk;
+    if (grouped) pl.pos[t] = (unsigned short)(j * ld + kk);
   }
-  pl.g2min = q.W ? lo2 : 0;
-  pl.n2 = q.W ? hi2 - lo2 + 1 : 0;
-  pl.g3min = q.W ? lo3 : 0;
-  pl.n3 = q.W ? hi3 - lo3 + 1 : 0;
-  for (int p = 0; p < q.n1; p++) pl.maxcnt = std::max(pl.maxcnt, pl.start[p + 1]);
-  // positions in the tile of the grouped form's first pass (used where that form is, and the tile fits)
-  const int pad = fft_band_tile_ld(N3) - N3;
-  for (int t = 0; t < q.W; t++) pl.pos[t] = (unsigned short)(pl.off[t] + pl.off[t] / N3 * pad);
-  for (int p = 0; p < q.n1; p++) pl.start[p + 1] += pl.start[p];
+}
+
+static void install_positions(DevKpt &q, const PlaneLists &pl) {
+  if (pl.pos.empty()) {
+    q.plane_pos.reset();
+    return;
+  }
+  q.plane_pos.alloc(pl.pos.size());
+  q.plane_pos.upload(pl.pos.data(), pl.pos.size());
 }
 
 static void install_planes(DevWF &d, DevKpt &q, const PlaneLists &pl) {
@@ -705,8 +716,7 @@ static void install_planes(DevWF &d, DevKpt &q, const PlaneLists &pl) {
   q.plane_start.upload(pl.start.data(), q.n1 + 1);
   q.plane_off.alloc(std::max(q.W, 1));
   q.plane_off.upload(pl.off.data(), q.W);
-  q.plane_pos.alloc(std::max(q.W, 1));
-  q.plane_pos.upload(pl.pos.data(), q.W);
+  install_positions(q, pl);
   q.off_N2 = d.N[1];
   q.off_N3 = d.N[2];
 }
@@ -1089,6 +1099,12 @@ static bool plane_geom(DevWF &d, int k, PlaneGeom &g) {
   g.n3 = q.n3;
   g.maxcnt = q.maxcnt;
   if (!choose_form(g)) return false;
+  if (g.grouped && !q.plane_pos.p) {
+    // the lists were made while a switch chose another form
+    PlaneLists pl;
+    plane_lists(d, q, pl);
+    install_positions(q, pl);
+  }
   for (int a = 0; a < 3 && g.grouped; a++)
     if (!d.tw2[g.order][a].p) upload_table(fft_band_table(g, a), d.tw2[g.order][a]);
   return true;
