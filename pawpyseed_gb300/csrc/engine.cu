@@ -2149,17 +2149,11 @@ int scratch_pieces(long long want, long long bytes_each, long long cap, long lon
   const long long budget = std::max(kScratchBytes, std::min(cap, free_bytes / 4));
   return (int)std::max(1LL, std::min(want, budget / std::max(1LL, bytes_each)));
 }
-// The same within one call of the library: the free memory is asked for once, and only where the pieces need more than
-// 1 GiB (asking takes 0.2 ms; per k-point it took a quarter of the density of 64 atoms on 120^3).
-struct ScratchBudget {
-  int count(long long want, long long bytes_each, long long cap) {
-    if (want * bytes_each > kScratchBytes && cap > kScratchBytes && free_ < 0) free_ = free_device_bytes();
-    return scratch_pieces(want, bytes_each, cap, std::max(0LL, free_));
-  }
-
- private:
-  long long free_ = -1;
-};
+// The same with what is free now (asked for, in 5 us, only where it can matter).
+static int scratch_count(long long want, long long bytes_each, long long cap) {
+  const bool ask = want * bytes_each > kScratchBytes && cap > kScratchBytes;
+  return scratch_pieces(want, bytes_each, cap, ask ? free_device_bytes() : 0);
+}
 
 // The real-space sphere tables of d's sites on grid N (built once per grid and site list).
 static AeTables &ae_tables(DevWF &d, const int *N, const int *labels, const double *coords) {
@@ -2444,7 +2438,7 @@ constexpr int kAeBatch = 16;
 
 // rho += sum of w |psi|^2 over the given bands of k-point kq (density.c:158-204).
 static void ae_density(DevWF &d, AeTables &t, int kq, const std::vector<int> &bands, const std::vector<double> &w,
-                       ScratchBudget &mem, DevBuf<float2> &g, double *rho) {
+                       DevBuf<float2> &g, double *rho) {
   const int ncell = t.N[0] * t.N[1] * t.N[2];
   std::vector<float2> ws;
   for (double v : w) ws.push_back(make_float2((float)v, (float)(v - (float)v)));
@@ -2453,8 +2447,8 @@ static void ae_density(DevWF &d, AeTables &t, int kq, const std::vector<int> &ba
   DevBuf<float4> bl;
   // runs of consecutive bands, in batches that the free memory holds
   const long long per_band = ncell * (long long)sizeof(float2) + rs_band_bytes(d, t, kq, ncell);
-  const size_t step = (size_t)mem.count(std::min<size_t>(kAeBatch, std::max<size_t>(1, bands.size())), per_band,
-                                        std::numeric_limits<long long>::max());
+  const size_t step = (size_t)scratch_count(std::min<size_t>(kAeBatch, std::max<size_t>(1, bands.size())), per_band,
+                                            std::numeric_limits<long long>::max());
   auto run_end = [&](size_t i) {
     size_t j = i + 1;
     while (j < bands.size() && bands[j] == bands[j - 1] + 1 && j - i < step) j++;
@@ -3093,7 +3087,7 @@ static void ae_grid_rows(DevWF &d, AeTables &t, int kq, int b0, int nb, float2 *
   if (ld > n3d)
     PAWPY_CUDA(cudaMemset2DAsync(rows + n3d, sizeof(float2) * ld, 0, sizeof(float2) * (ld - n3d), nb, stream()));
   DevBuf<float4> bl;
-  const int step = scratch_pieces(nb, rs_band_bytes(d, t, kq, ld), kScratchBytes, 0);
+  const int step = scratch_count(nb, rs_band_bytes(d, t, kq, ld), kScratchBytes);
   for (int b = 0; b < nb; b += step) {
     const int n = std::min(step, nb - b);
     rs_grids(d, t, kq, b0 + b, n, rows + (size_t)b * ld, ld);
@@ -3125,7 +3119,7 @@ static void realspace_overlaps(pswf_t *wf_S, pswf_t *wf_R, const int *fftg, cons
   const int nk = S.nk, nbR = R.nband;
   const double scale = S.vol / (double)n3d;
   const long long per_k = (long long)(ns + nbR) * ld * (long long)sizeof(float2);
-  const int kb = ScratchBudget().count(nk, per_k, kAeOverlapBytes);
+  const int kb = scratch_count(nk, per_k, kAeOverlapBytes);
   DevBuf<float2> gS((size_t)kb * ns * ld), gR((size_t)kb * nbR * ld), o((size_t)nk * ns * nbR);
   for (int k0 = 0; k0 < nk; k0 += kb) {
     const int n = std::min(kb, nk - k0);
@@ -3182,11 +3176,10 @@ void ae_state_density(double *P, int BAND_NUM, int KPOINT_NUM, pswf_t *wf, int *
   AeTables &t = ae_tables(d, fftg, labels, coords);
   const long long n3d = (long long)fftg[0] * fftg[1] * fftg[2];
   ensure_projections(d);
-  ScratchBudget mem;
   DevBuf<float2> g;
   DevBuf<double> rho(n3d);
   rho.upload(P, n3d);
-  ae_density(d, t, KPOINT_NUM, {BAND_NUM}, {1.0}, mem, g, rho.p);
+  ae_density(d, t, KPOINT_NUM, {BAND_NUM}, {1.0}, g, rho.p);
   rho.download(P, n3d);
   sync();
   PAWPY_API_END()
@@ -3201,7 +3194,6 @@ void ae_chg_density(double *P, pswf_t *wf, int *fftg, int *labels, double *coord
   AeTables &t = ae_tables(d, fftg, labels, coords);
   const long long n3d = (long long)fftg[0] * fftg[1] * fftg[2];
   ensure_projections(d);
-  ScratchBudget mem;
   DevBuf<float2> g;
   DevBuf<double> rho(n3d);
   rho.upload(P, n3d);
@@ -3217,7 +3209,7 @@ void ae_chg_density(double *P, pswf_t *wf, int *fftg, int *labels, double *coord
         wk.push_back(wf->kpts[k]->weight * bd->occ * spin_mult);
       }
     }
-    ae_density(d, t, k, occ, wk, mem, g, rho.p);
+    ae_density(d, t, k, occ, wk, g, rho.p);
   }
   rho.download(P, n3d);
   sync();
@@ -3250,7 +3242,6 @@ void ncl_ae_chg_density(double *P, pswf_t *wf, int *fftg, int *labels, double *c
   AeTables &t = ae_tables(d, fftg, labels, coords);
   const long long n3d = (long long)fftg[0] * fftg[1] * fftg[2];
   ensure_projections(d);
-  ScratchBudget mem;
   DevBuf<float2> g;
   DevBuf<double> rho(n3d);
   rho.upload(P, n3d);
@@ -3266,7 +3257,7 @@ void ncl_ae_chg_density(double *P, pswf_t *wf, int *fftg, int *labels, double *c
           wk.push_back(wf->kpts[k]->weight * bd->occ);
         }
     }
-    ae_density(d, t, k, occ, wk, mem, g, rho.p);
+    ae_density(d, t, k, occ, wk, g, rho.p);
   }
   rho.download(P, n3d);
   sync();
