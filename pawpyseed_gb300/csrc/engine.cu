@@ -2395,27 +2395,39 @@ static const float2 *proj_rows(DevWF &d, int kq, int b0) {
   return d.P.p + ((size_t)kq * d.nband + b0) * d.proj.Ptot;
 }
 
-// The Bloch factors of k-point kq on the grid of t (scale included): f(slab) for the whole grid, or for one slab
-// of the first axis after another where the grid's table (16 bytes per cell) would be larger than kBlochBytes. buf keeps
-// the whole grid's for the k-point's other calls.
+// The Bloch factors of k-point kq on the grid of t (scale included), 16 bytes per cell: whole, built once, or
+// in slabs of the first axis where a table would be larger than kBlochBytes.
 constexpr long long kBlochBytes = 256LL << 20;
-template <typename F>
-static void with_bloch(DevWF &d, AeTables &t, int kq, DevBuf<float4> &buf, F &&f) {
-  const int *N = t.N;
-  const long long plane = (long long)N[1] * N[2];
-  const int nx = (int)std::max(1LL, std::min<long long>(N[0], kBlochBytes / (plane * (long long)sizeof(float4))));
-  if (kpoint_is_gamma(d.kp[kq])) {
-    f(BlochSlab{nullptr, 0, N[0]});
-    return;
+struct BlochFactors {
+  BlochFactors(DevWF &d, AeTables &t, int kq) : d_(d), t_(t), kq_(kq) {
+    const int *N = t.N;
+    const long long plane = (long long)N[1] * N[2];
+    nx_ = (int)std::max(1LL, std::min<long long>(N[0], kBlochBytes / (plane * (long long)sizeof(float4))));
+    if (kpoint_is_gamma(d.kp[kq])) return;
+    buf_.alloc((size_t)nx_ * plane);
+    if (nx_ == N[0]) fill({buf_.p, 0, nx_});
   }
-  const bool whole = nx == N[0], built = whole && buf.n;
-  if (!buf.n) buf.alloc((size_t)nx * plane);
-  for (int x0 = 0; x0 < N[0]; x0 += nx) {
-    const BlochSlab slab{buf.p, x0, std::min(nx, N[0] - x0)};
-    if (!built) launch_bloch_table(N, slab, d.kp[kq].kfrac, std::pow(d.vol, -0.5), buf.p);
-    f(slab);
+  // f(slab) over the whole grid
+  template <typename F>
+  void apply(F &&f) {
+    const int N1 = t_.N[0];
+    if (!buf_.n || nx_ == N1) return f(BlochSlab{buf_.p, 0, N1});
+    for (int x0 = 0; x0 < N1; x0 += nx_) {
+      const BlochSlab slab{buf_.p, x0, std::min(nx_, N1 - x0)};
+      fill(slab);
+      f(slab);
+    }
   }
-}
+
+ private:
+  void fill(const BlochSlab &slab) {
+    launch_bloch_table(t_.N, slab, d_.kp[kq_].kfrac, std::pow(d_.vol, -0.5), buf_.p);
+  }
+  DevWF &d_;
+  AeTables &t_;
+  int kq_, nx_;
+  DevBuf<float4> buf_;
+};
 
 // All-electron states of bands [b0, b0 + nb) of k-point kq to host x (realspace_state,
 // density.c:245-310).
@@ -2425,8 +2437,7 @@ static void ae_states(DevWF &d, AeTables &t, int kq, int b0, int nb, pawpy_c128 
   DevBuf<float2> g((size_t)nb * n3d);
   rs_grids(d, t, kq, b0, nb, g.p, n3d);
   DevBuf<double2> o((size_t)nb * n3d);
-  DevBuf<float4> bl;
-  with_bloch(d, t, kq, bl, [&](const BlochSlab &slab) {
+  BlochFactors(d, t, kq).apply([&](const BlochSlab &slab) {
     launch_ae_states(t.view, proj_rows(d, kq, b0), d.proj.Ptot, kq, slab, std::pow(d.vol, -0.5), g.p, n3d, nb, t.N, o.p);
   });
   o.download(reinterpret_cast<double2 *>(x), o.n);
@@ -2444,7 +2455,6 @@ static void ae_density(DevWF &d, AeTables &t, int kq, const std::vector<int> &ba
   for (double v : w) ws.push_back(make_float2((float)v, (float)(v - (float)v)));
   DevBuf<float2> wd(std::max<size_t>(1, ws.size()));
   wd.upload(ws.data(), ws.size());
-  DevBuf<float4> bl;
   // runs of consecutive bands, in batches that the free memory holds
   const long long per_band = ncell * (long long)sizeof(float2) + rs_band_bytes(d, t, kq, ncell);
   const size_t step = (size_t)scratch_count(std::min<size_t>(kAeBatch, std::max<size_t>(1, bands.size())), per_band,
@@ -2459,12 +2469,14 @@ static void ae_density(DevWF &d, AeTables &t, int kq, const std::vector<int> &ba
     j = run_end(i);
     longest = std::max(longest, j - i);
   }
+  if (longest == 0) return;
   if (g.n < longest * ncell) g.alloc(longest * ncell);
+  BlochFactors bloch(d, t, kq);
   for (size_t i = 0, j; i < bands.size(); i = j) {
     j = run_end(i);
     const int nb = (int)(j - i);
     rs_grids(d, t, kq, bands[i], nb, g.p, ncell);
-    with_bloch(d, t, kq, bl, [&](const BlochSlab &slab) {
+    bloch.apply([&](const BlochSlab &slab) {
       launch_ae_density(t.view, proj_rows(d, kq, bands[i]), d.proj.Ptot, kq, slab, std::pow(d.vol, -0.5), g.p, ncell, nb,
                         t.N, wd.p + i, rho);
     });
@@ -3086,12 +3098,12 @@ static void ae_grid_rows(DevWF &d, AeTables &t, int kq, int b0, int nb, float2 *
   ensure_projections(d);
   if (ld > n3d)
     PAWPY_CUDA(cudaMemset2DAsync(rows + n3d, sizeof(float2) * ld, 0, sizeof(float2) * (ld - n3d), nb, stream()));
-  DevBuf<float4> bl;
+  BlochFactors bloch(d, t, kq);
   const int step = scratch_count(nb, rs_band_bytes(d, t, kq, ld), kScratchBytes);
   for (int b = 0; b < nb; b += step) {
     const int n = std::min(step, nb - b);
     rs_grids(d, t, kq, b0 + b, n, rows + (size_t)b * ld, ld);
-    with_bloch(d, t, kq, bl, [&](const BlochSlab &slab) {
+    bloch.apply([&](const BlochSlab &slab) {
       launch_ae_store(t.view, proj_rows(d, kq, b0 + b), d.proj.Ptot, kq, slab, std::pow(d.vol, -0.5),
                       rows + (size_t)b * ld, ld, n, t.N);
     });
