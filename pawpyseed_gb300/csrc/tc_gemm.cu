@@ -571,6 +571,8 @@ void run_tc(const GemmBatch *batches_dev, const std::vector<GemmBatch> &hb, int 
       tc_tuned()[key] = choice;
     }
   }
+  // (a choice made for a longer K of the same key may have more splits than this K's workspace holds)
+  choice.splits = std::min(choice.splits, max_splits);
   run(choice);
   status_readback(st, "tensor-core overlap: a pipeline wait timed out");
   if (info) {
