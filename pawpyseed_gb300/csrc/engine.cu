@@ -1149,7 +1149,7 @@ static long long l2_bytes() {
 // Issues the first FFT pass of every band and k-point on the auxiliary stream
 // (each k-point after its coefficient upload), so that it runs while the host
 // builds the sphere tables; project_bands then runs the second pass from Hall.
-// Only for grids of the register kernels, an H of at most kEarlyPlanesBytes,
+// Only for grids that a fast form covers (choose_form), an H of at most kEarlyPlanesBytes,
 // and k-points whose H exceeds the L2 cache anyway (measured: at 36x45x50 a
 // k-point's 77 MB of H stays in L2 between the passes of the interleaved form,
 // and the early form made the second pass 2.4 times slower). Threads on a

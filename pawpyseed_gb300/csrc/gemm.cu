@@ -11,17 +11,18 @@
 
 namespace pawpy {
 
-// One output tile per CTA of four warps. A thread holds RM rows (basis bands) x RN columns (defect
-// bands); its sums are packed FP32 pairs of two neighbouring rows, so that the four multiply-adds of a
-// complex product of two rows are four FFMA2. Chunks of 16 k go from global memory through registers
-// into planar shared tiles [k][row] of re, im, -im (A) and re, im (B), double-buffered; a thread's rows
+// One output tile per CTA (64 x 64: four warps; 32 x 32: two). A thread holds RM rows (basis bands) x RN
+// columns (defect bands); its sums are packed FP32 pairs of two neighbouring rows, so that the four
+// multiply-adds of a complex product of two rows are four FFMA2. Chunks of 16 k go from global memory
+// through registers into planar shared tiles [k][row] of re and im, double-buffered; a thread's rows
 // of one plane are 16-byte loads that the warp shares (one wavefront each).
 //
-// Bound: the FP32 pipes. Per k a thread of the 64 x 64 tile issues 64 FFMA2 (128 of the pipe's cycles)
-// beside 8 shared loads and 16 moves, so the pipes, not the issue slots, are full; the form with scalar
-// multiply-adds and 4 x 4 sums per thread reached 32 TFLOP/s at 300 x 250 x 23,056 (0.44 ms with its
-// reduction). Every sum keeps its order: k ascending within a split, acc_r + a.y b.y + a.x b.x and
-// acc_i - a.y b.x + a.x b.y.
+// Bound: shared-memory reads beside the FP32 pipe. Per k a thread of the 64 x 64 tile issues 64 FFMA2 (128 of
+// the pipe's cycles) and 6 shared loads; 168 registers leave three CTAs per SM. At 300 x 250 x 23,056 (22
+// splits, 291 us, 47 TFLOP/s) the FMA pipe is 65% and the shared-memory path 77% busy, and the warps wait
+// mostly for the loads (short scoreboard). The form with scalar multiply-adds and 4 x 4 sums per thread reached
+// 32 TFLOP/s there (0.44 ms with its reduction, now 0.297). Every sum keeps its order: k ascending within a
+// split, acc_r + a.y b.y + a.x b.x and acc_i - a.y b.x + a.x b.y.
 namespace {
 
 constexpr int BK = 16;

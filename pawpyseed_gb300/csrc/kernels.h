@@ -77,7 +77,7 @@ void launch_fft_x_grid(const float2 *H, const PlaneGeom &g, float2 *grid, int b0
 void launch_flatten_pick(const GatherSeg *segs, const int *base, int nsegs, int nkp, int N3, const int *rowoff,
                          const int *coloff, long long kb_words, PickList &pl);
 // The two passes for the other grids whose lengths split into two groups and whose planes fit in
-// shared memory (fft_band.cuh); fft_band_supported tells whether g is one.
+// shared memory beside the static masks (fft_band.cuh); fft_band_supported tells whether g is one.
 bool fft_band_supported(const PlaneGeom &g);
 // row length of the first pass's tile of coefficients
 int fft_band_tile_ld(int n3);

@@ -29,10 +29,9 @@ constexpr long long kNoallocMaxOutput = 4LL << 20;  // 4,194,304 values = 32 MiB
 static __device__ __align__(256) float2 g_noalloc_scratch[kNoallocMaxOutput];
 
 namespace {
-// split-K factor: enough CTAs for two waves on the device's SMs, at least 32 K-chunks of 16 per split
-// As many splits as fill the SMs once with the tile's three resident CTAs each: at 300 x 250 x 23,056,
-// 22 splits of 20 tiles (2.9 CTAs on every SM); with the 16 of two per SM some SMs hold three and the
-// rest wait.
+// split-K factor: as many splits as fill the SMs once with the tile's three resident CTAs each, at least 32
+// K-chunks of 16 per split. At 300 x 250 x 23,056: 22 splits of 20 tiles (2.9 CTAs on every SM); with the 16
+// of two per SM some SMs hold three and the rest wait.
 int noalloc_splits(int M, int N, int K, int sms) {
   int tiles = ceil_div(M, 64) * ceil_div(N, 64);
   int s = std::max(1, 3 * sms / tiles);
